@@ -243,11 +243,17 @@ k_t2_interp(const cpx<R> *__restrict__ grid, float *__restrict__ sino,
 // the weights stay in registers.
 // ---------------------------------------------------------------------------
 // ES kernel weight exp(beta (sqrt(1 - z^2) - 1)) for |z| < 1, else 0, on the
-// fast hardware square root and exponential (relative error ~1e-6)
-__device__ __forceinline__ float es_weight_fast(float z, float beta) {
-    const float q = 1.f - z * z;
-    return q > 0.f ? __expf(beta * (q * rsqrtf(q) - 1.f)) : 0.f;
+// hardware's approximate square root and 2^x (relative error ~1e-6);
+// beta2 = beta log2(e).  The .ftz forms need no scaling steps around them: a
+// q below 2^-126 is as good as 0
+__device__ __forceinline__ float es_weight_fast(float z, float beta2) {
+    const float q = fmaf(-z, z, 1.f);
+    float s, f;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(q));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(fmaf(beta2, s, -beta2)));
+    return q > 0.f ? f : 0.f;
 }
+constexpr float LOG2E = 1.44269504088896340736f;
 
 __host__ __device__ constexpr int interp_pitch(int ts, int w) { return (ts + w) & ~1; }
 
@@ -280,14 +286,15 @@ k_t2_interp_tile(const c32 *__restrict__ grid, c32 *__restrict__ cpts,
     cp_async_wait_all();
     __syncthreads();
     constexpr float inv_half = 2.f / (float)W;
+    const float beta2 = beta * LOG2E;
     for (int i = threadIdx.x; i < sb.count; i += INTERP_THREADS) {
         const InterpEntry e = load_entry(entries, sb.start + i);
         const int pt = e.pt;
         float wx[W], wy[W];
 #pragma unroll
         for (int t = 0; t < W; ++t) {
-            wx[t] = es_weight_fast(((float)t - e.fx) * inv_half, beta);
-            wy[t] = es_weight_fast(((float)t - e.fy) * inv_half, beta);
+            wx[t] = es_weight_fast(((float)t - e.fx) * inv_half, beta2);
+            wy[t] = es_weight_fast(((float)t - e.fy) * inv_half, beta2);
         }
         // the point's first tap inside the region (its tile holds it)
         const c32 *base = reg + e.off;
@@ -356,6 +363,7 @@ k_t2_interp_lanes(const c32 *__restrict__ grid, c32 *__restrict__ cpts,
     const int lane = threadIdx.x & 31, gbase = lane & 16;
     const int gl = lane & 15, b = gl >> 1, h = gl & 1;
     constexpr float inv_half = 2.f / (float)W;
+    const float beta2 = beta * LOG2E;
     // i0 is uniform over the warp (its two groups take points i0, i0 + 1), so
     // every lane reaches every shuffle
     for (int i0 = (threadIdx.x >> 5) * 2; i0 < sb.count; i0 += NG) {
@@ -364,7 +372,7 @@ k_t2_interp_lanes(const c32 *__restrict__ grid, c32 *__restrict__ cpts,
         const InterpEntry e = load_entry(entries, sb.start + (act ? i : i0));
         const float f = gl < W ? e.fx : e.fy;
         const int tk = gl < W ? gl : gl - W;
-        const float wl = gl < 2 * W ? es_weight_fast(((float)tk - f) * inv_half, beta) : 0.f;
+        const float wl = gl < 2 * W ? es_weight_fast(((float)tk - f) * inv_half, beta2) : 0.f;
         float wx[W], wy[KY];
 #pragma unroll
         for (int t = 0; t < W; ++t) wx[t] = __shfl_sync(0xffffffffu, wl, gbase + t);
@@ -513,208 +521,264 @@ __global__ void k_zero_tiles(cpx<R> *__restrict__ grid, const int *__restrict__ 
 
 // ---------------------------------------------------------------------------
 // type 1, pass 1 on bands (register-FFT path, column-major grid
-// grid[b][x][y]): one warp per chunk of a band's point list.  Lane
-// (rho, c) = (lane / 8, lane % 8) takes tap (rho - dy0, c) of the current
-// point, i.e. cell (rho, dx0 + c) of the band.  The accumulator holds
-// [line][row][BAND_RS] complex values with BAND_RS = 40 (= 8 mod 16), so a
-// point's 32 lane cells fill the 16 bank pairs twice each, the minimum for
-// 8-byte accesses; it belongs to the warp alone, so plain shared-memory adds
-// suffice, __syncwarp ordering consecutive points.  Each of the first 16
-// lanes evaluates one kernel weight (lanes 0-7 the columns, 8-15 the rows),
-// shuffled to the lanes that use it.  Entries and their point values are
-// loaded two and one points ahead.
+// grid[b][x][y]).  A band is 8 x 8 cells; a warp walks chunks of the bands'
+// point lists (chunk i, i + warps, ...) with the band in registers: lane
+// (g, c) = (lane / 8, lane % 8) owns column c of the band, for two lines and
+// eight rows (LPL = 2: chunks of 5 .. 8 lines), one line and eight rows
+// (RS = 1: 3 or 4 lines), four rows (RS = 2: two lines) or two rows (RS = 4:
+// one line).  Cells outside an entry's footprint get weight zero, so every
+// entry runs the same straight-line code: no branch on its position, no
+// shared-memory accumulators, no atomics inside a band.
+//
+// The list is taken 32 entries at a time.  First lane e takes entry e alone:
+// it evaluates the band's eight column and eight row weights for it into a
+// record in the warp's shared memory.  Then the warp walks the 32 records: a
+// lane reads its column weight, its rows' weights and its lines' values and
+// adds to its cells with paired FMAs (fma.rn.f32x2 on two rows).  Entries
+// are loaded two batches ahead and their point values one batch ahead
+// (cp.async, one copy per line and entry: neighbouring entries are
+// neighbouring points of a ray and share sectors), across chunk borders.
+//
+// What bounds it: shared-memory wavefronts and issue (ncu, 16 slices of
+// 1536^2, 1500 angles: L1 data pipe 70 %, issue 55 %, FMA pipe about half;
+// 48 instructions and 40 FMA-pipe cycles per entry for eight lines).  Measured
+// there, spreading alone: 1473 us with 32 x 4 bands, a switch on the column
+// (compiled to a tree of branches) and one shuffled weight per lane; 868 with
+// batched weights; 569 in this form.  2908^2, 1969 angles: 3608 -> 1949 us;
+// 5 slices of 1001^2: 383 -> 126 us.  Bands are numbered down the columns and
+// stored by whole sectors: row-major numbering and 16-byte stores took 693
+// and 2443 us.  Walking runs of several sparse bands per batch issued 16 %
+// fewer instructions but was slower (671 us).
 // ---------------------------------------------------------------------------
-constexpr int BAND_RS = BAND_W + 8;
-constexpr int BAND_WARPS = 8;
-static_assert(BAND_H * 8 == 32, "a band row group is one warp of 8-lane rows");
+constexpr int BAND_WARPS = 4;
+constexpr int BAND_LINES = 8;
+// CTAs per SM: 16 warps of at most 128 registers for two lines per lane, else
+// 24 of at most 85
+constexpr int band_ctas(int lpl) { return lpl == 2 ? 4 : 6; }
+static_assert(BAND_W == 8 && BAND_H == 8, "lane (g, c) owns column c of an 8 x 8 band");
+static_assert(NB_MAX <= BAND_LINES, "a chunk's lines fit a warp");
+// an entry's record; 80 bytes put eight consecutive records on distinct
+// 16-byte bank groups
+struct __align__(16) BandRec {
+    float wx[BAND_W], wy[BAND_H];
+    float pad[4];
+};
+static_assert(sizeof(BandRec) == 80, "record stride");
+constexpr int BAND_VS = BAND_LINES + 2;  // value row stride (complex), 16-byte aligned rows
+struct BandWarp {
+    BandRec rec[32];
+    c32 val[2][32 * BAND_VS];
+};
 
-template <int NB>
-__global__ void __launch_bounds__(BAND_WARPS * 32, NB <= 3 ? 6 : NB == 4 ? 5 : 4)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma_x2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul_x2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pack_x2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpack_x2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+// position in the stream of a warp's batches: chunk ci (descriptor ch), its
+// entries base .. base + 31; chn is the warp's next chunk, loaded ahead
+struct BandPos {
+    int ci, base;
+    BandChunk ch, chn;
+};
+
+template <int W, int LPL, int RS>
+__global__ void __launch_bounds__(BAND_WARPS * 32, band_ctas(LPL))
 k_spread_band(const c32 *__restrict__ cpts, c32 *__restrict__ grid,
-              const BandEntry *__restrict__ ent, const BandChunk *__restrict__ chunks,
-              int nchunk, int nf, int npts, int w, float beta) {
-    constexpr int nb = NB;
+              const BandEntry *__restrict__ ent, const BandChunk *__restrict__ chunks, int nchunk,
+              int nf, int npts, float beta, int nl) {
+    static_assert(LPL == 1 || RS == 1, "two lines per lane only with all rows");
+    constexpr int RP = BAND_H / RS;  // rows per lane
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int ci = blockIdx.x * BAND_WARPS + wid;
-    if (ci >= nchunk) return;  // no block-wide barrier below
-    constexpr int PLANE = BAND_H * BAND_RS;  // one line's complex cells
-    c32 *acc = reinterpret_cast<c32 *>(smem_raw) + (size_t)wid * nb * PLANE;
-    for (int q = lane; q < nb * PLANE; q += 32) acc[q] = mk<float>(0.f, 0.f);
-    const BandChunk ch = chunks[ci];
-    const int rho = lane >> 3, c = lane & 7;
-    const float inv_half = 2.f / (float)w;
-    const bool wlane = lane < 16 && (lane & 7) < w;  // evaluates weight (lane & 7)
-    auto load_vals = [&](const BandEntry &e, c32 *v) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-            v[b] = cpts ? cpts[(size_t)b * npts + e.pt] : mk<float>(1.f, 0.f);
+    const int nwarps = gridDim.x * BAND_WARPS, w0 = blockIdx.x * BAND_WARPS + wid;
+    if (w0 >= nchunk) return;  // no block-wide barrier below
+    BandWarp &sm = reinterpret_cast<BandWarp *>(smem_raw)[wid];
+    const int c = lane & 7, g = lane >> 3;
+    const int line = LPL == 2 ? 2 * g : g / RS;  // this lane's (first) line
+    const int row = (g % RS) * RP;               // and first row
+    constexpr float inv_half = 2.f / (float)W;
+    const float beta2 = beta * LOG2E;
+    auto load_chunk = [&](int i) {
+        if (i >= nchunk) return BandChunk{0, 0, 0, 0};
+        const int4 q = __ldg(reinterpret_cast<const int4 *>(chunks) + i);
+        return BandChunk{q.x, q.y, q.z, q.w};
     };
-    __syncwarp();
-    BandEntry en{}, nx{};
-    c32 v[NB], vn[NB];
-    if (ch.count > 0) {
-        en = ent[ch.start];
-        load_vals(en, v);
-    }
-    if (ch.count > 1) nx = ent[ch.start + 1];
-    for (int e = 0; e < ch.count; ++e) {
-        BandEntry nn{};
-        if (e + 2 < ch.count) nn = ent[ch.start + e + 2];
-        if (e + 1 < ch.count) load_vals(nx, vn);
-        const int dx0 = (int)(short)(en.dxy & 0xffff), dy0 = en.dxy >> 16;
-        // lane l < 8: column weight of tap l; 8 <= l < 16: row weight of tap l - 8
-        const float zf = ((float)(lane & 7) - (lane < 8 ? en.fx : en.fy)) * inv_half;
-        const float f = wlane ? es_weight_fast(zf, beta) : 0.f;
-        const int ty = rho - dy0, col = dx0 + c;
-        const float wxc = __shfl_sync(0xffffffffu, f, c);
-        const float wyr = __shfl_sync(0xffffffffu, f, 8 + (ty & 7));
-        if (c < w && ty >= 0 && ty < w && col >= 0 && col < BAND_W) {
-            const float wgt = wxc * wyr;
-            c32 *a = acc + rho * BAND_RS + col;
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                c32 t = a[b * PLANE];
-                t.x = fmaf(v[b].x, wgt, t.x);
-                t.y = fmaf(v[b].y, wgt, t.y);
-                a[b * PLANE] = t;
-            }
+    auto next = [&](const BandPos &p) {
+        BandPos n = p;
+        n.base += 32;
+        if (n.base >= n.ch.count) {
+            n.ci += nwarps;
+            n.base = 0;
+            n.ch = p.chn;
+            n.chn = load_chunk(n.ci + nwarps);
         }
-        __syncwarp();
-        en = nx;
-        nx = nn;
+        return n;
+    };
+    auto on = [&](const BandPos &p) { return p.base + lane < p.ch.count; };
+    auto load_ent = [&](const BandPos &p) {
+        if (!on(p)) return BandEntry{0, 0, 0.f, 0.f};
+        const int4 q = __ldg(reinterpret_cast<const int4 *>(ent) + p.ch.start + p.base + lane);
+        return BandEntry{q.x, q.y, __int_as_float(q.z), __int_as_float(q.w)};
+    };
+    // this lane's entry's values of all lines into value buffer buf
+    constexpr int NLX = LPL == 2 ? BAND_LINES : 4 / RS;  // most lines of this shape
+    auto fetch_vals = [&](const BandEntry &e, bool act, int buf) {
+        c32 *dst = sm.val[buf] + lane * BAND_VS;
+        const c32 *src = cpts + e.pt;
 #pragma unroll
-        for (int b = 0; b < NB; ++b) v[b] = vn[b];
-    }
-    // store the band: lane (column lane / 4 + 8 k, row lane % 4); the four
-    // rows of a column are 32 contiguous bytes of the column-major grid
-    const int nbx = nf / BAND_W;
-    const int bx = ch.band % nbx, by = ch.band / nbx;
-    const int r = lane & 3;
-    for (int b = 0; b < nb; ++b)
-        for (int k = 0; k < BAND_W / 8; ++k) {
-            const int cc = (lane >> 2) + 8 * k;
-            const c32 val = acc[b * PLANE + r * BAND_RS + cc];
-            c32 *dst = grid + ((size_t)b * nf + bx * BAND_W + cc) * nf + by * BAND_H + r;
-            if (ch.shared) {
-                atomicAdd(&dst->x, val.x);
-                atomicAdd(&dst->y, val.y);
+        for (int q = 0; q < NLX; ++q) {
+            if (act && q < nl) {
+                if (cpts) cp_async8(dst + q, src);
+                else dst[q] = mk<float>(1.f, 0.f);
+            }
+            src += npts;
+        }
+        cp_async_commit();
+    };
+    f32x2 acc[RP / 2][LPL][2];  // [row pair][line][re, im]
+    auto clear = [&]() {
+#pragma unroll
+        for (int r = 0; r < RP / 2; ++r)
+#pragma unroll
+            for (int l = 0; l < LPL; ++l) acc[r][l][0] = acc[r][l][1] = 0ull;
+    };
+    clear();
+    // cur: the batch being added; nx: its successor, entries loaded; fu: the
+    // one after, entries requested
+    BandPos cur{w0, 0, load_chunk(w0), load_chunk(w0 + nwarps)};
+    BandEntry ecur = load_ent(cur);
+    BandPos nx = next(cur);
+    BandEntry enx = load_ent(nx);
+    fetch_vals(ecur, on(cur), 0);
+    for (int buf = 0; cur.ci < nchunk; buf ^= 1) {
+        const BandPos fu = next(nx);
+        const BandEntry efu = load_ent(fu);
+        const int m = min(32, cur.ch.count - cur.base);
+        // z of cell q: (q - dx0 - fx) 2 / W, the integer part exact
+        const float dx0 = (float)(int)(short)(ecur.dxy & 0xffff), dy0 = (float)(ecur.dxy >> 16);
+        const float ox = ecur.fx * inv_half, oy = ecur.fy * inv_half;
+        BandRec rec;
+#pragma unroll
+        for (int q = 0; q < BAND_W; ++q) rec.wx[q] = es_weight_fast(fmaf((float)q - dx0, inv_half, -ox), beta2);
+#pragma unroll
+        for (int q = 0; q < BAND_H; ++q) rec.wy[q] = es_weight_fast(fmaf((float)q - dy0, inv_half, -oy), beta2);
+        __syncwarp();  // the last batch has been read
+        float4 *rd = reinterpret_cast<float4 *>(&sm.rec[lane]);
+        rd[0] = make_float4(rec.wx[0], rec.wx[1], rec.wx[2], rec.wx[3]);
+        rd[1] = make_float4(rec.wx[4], rec.wx[5], rec.wx[6], rec.wx[7]);
+        rd[2] = make_float4(rec.wy[0], rec.wy[1], rec.wy[2], rec.wy[3]);
+        rd[3] = make_float4(rec.wy[4], rec.wy[5], rec.wy[6], rec.wy[7]);
+        fetch_vals(enx, on(nx), buf ^ 1);
+        cp_async_wait_prev();
+        __syncwarp();  // records and this batch's values visible
+        const c32 *vals = sm.val[buf] + (line < nl ? line : 0);
+#pragma unroll 4
+        for (int e = 0; e < m; ++e) {
+            const BandRec &q = sm.rec[e];
+            const float wx = q.wx[c];
+            const f32x2 wx2 = pack_x2(wx, wx);
+            f32x2 w[RP / 2];
+            if constexpr (RP >= 4) {
+#pragma unroll
+                for (int r = 0; r < RP / 4; ++r) {
+                    const ulonglong2 p = *reinterpret_cast<const ulonglong2 *>(&q.wy[row + 4 * r]);
+                    w[2 * r] = mul_x2(wx2, p.x);
+                    w[2 * r + 1] = mul_x2(wx2, p.y);
+                }
             } else {
-                *dst = val;
+                w[0] = mul_x2(wx2, *reinterpret_cast<const f32x2 *>(&q.wy[row]));
+            }
+            c32 v[LPL];
+            if constexpr (LPL == 2) {
+                const float4 f = *reinterpret_cast<const float4 *>(vals + e * BAND_VS);
+                v[0] = mk<float>(f.x, f.y);
+                v[1] = mk<float>(f.z, f.w);
+            } else {
+                v[0] = vals[e * BAND_VS];
+            }
+#pragma unroll
+            for (int l = 0; l < LPL; ++l) {
+                const f32x2 vx = pack_x2(v[l].x, v[l].x), vy = pack_x2(v[l].y, v[l].y);
+#pragma unroll
+                for (int r = 0; r < RP / 2; ++r) {
+                    acc[r][l][0] = fma_x2(vx, w[r], acc[r][l][0]);
+                    acc[r][l][1] = fma_x2(vy, w[r], acc[r][l][1]);
+                }
             }
         }
-}
-
-// ---------------------------------------------------------------------------
-// type 1, pass 1 on bands with the accumulator in registers (chunks of 8
-// slices): lane (b, r) = (lane / 4, lane % 4) owns row r of the band for
-// slice b, 32 complex cells in registers, so a point adds its taps with no
-// shared-memory traffic.  Every lane takes the point's value of its own
-// slice, its row weight and the W column weights (evaluated by 2W lanes and
-// shuffled, as in k_spread_band) and adds to the cells dx0 .. dx0+W-1 of its
-// row: a switch on dx0 (the same for the whole warp, one point at a time)
-// whose cases name the cells at compile time.  Same lists, chunks, weights,
-// products and per-cell summation order as k_spread_band, so the grids are
-// bit-identical; a warp issues about a quarter of the instructions per point.
-// ---------------------------------------------------------------------------
-template <int W, int D>
-__device__ __forceinline__ void band_row_add(float2 (&acc)[BAND_W], const float (&wx)[8], float wyr,
-                                             c32 v) {
+        if (nx.ci != cur.ci) {
+            // the chunk is done: column c of the band, rows row .. row + RP - 1
+            // (contiguous in the column-major grid, two cells per 16 bytes)
+            const int nby = nf / BAND_H;
+            const int bx = cur.ch.band / nby, by = cur.ch.band - bx * nby;
+            auto cells = [&](int r, int l) {
+                const float2 re = unpack_x2(acc[r][l][0]), im = unpack_x2(acc[r][l][1]);
+                return make_float4(re.x, im.x, re.y, im.y);
+            };
+            auto put = [&](float4 *dst, float4 v, int l) {
+                if (line + l >= nl) return;
+                if (cur.ch.shared) atomicAdd(dst, v);
+                else *dst = v;
+            };
 #pragma unroll
-    for (int c = 0; c < W; ++c) {
-        const int k = D + c;
-        if (k >= 0 && k < BAND_W) {
-            const float wgt = wx[c] * wyr;
-            acc[k].x = fmaf(v.x, wgt, acc[k].x);
-            acc[k].y = fmaf(v.y, wgt, acc[k].y);
-        }
-    }
-}
-
-constexpr int BAND8_NB = 8;
-static_assert(BAND8_NB * BAND_H == 32, "a warp's lanes are the chunk's slices x the band's rows");
-
-template <int W>
-__global__ void __launch_bounds__(BAND_WARPS * 32, 2)
-k_spread_band8(const c32 *__restrict__ cpts, c32 *__restrict__ grid,
-               const BandEntry *__restrict__ ent, const BandChunk *__restrict__ chunks, int nchunk,
-               int nf, int npts, float beta) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int ci = blockIdx.x * BAND_WARPS + wid;
-    if (ci >= nchunk) return;  // no block-wide barrier below
-    const int b = lane >> 2, r = lane & 3;
-    float2 acc[BAND_W];
+            for (int l = 0; l < LPL; ++l) {
+                c32 *col = grid + ((size_t)(line + l < nl ? line + l : 0) * nf + bx * BAND_W + c) * nf +
+                           by * BAND_H + row;
+                if constexpr (RP == 2) {
+                    put(reinterpret_cast<float4 *>(col), cells(0, l), l);
+                } else {
+                    // lanes c and c ^ 1 trade a row pair, so that each store
+                    // writes whole 32-byte sectors: first the even column's
+                    // four rows, then the odd one's
+                    const bool odd = c & 1;
 #pragma unroll
-    for (int k = 0; k < BAND_W; ++k) acc[k] = make_float2(0.f, 0.f);
-    const BandChunk ch = chunks[ci];
-    const float inv_half = 2.f / (float)W;
-    const bool wlane = lane < 16 && (lane & 7) < W;  // evaluates weight (lane & 7)
-    auto load_val = [&](const BandEntry &e) {
-        return cpts ? cpts[(size_t)b * npts + e.pt] : mk<float>(1.f, 0.f);
-    };
-    BandEntry en{}, nx{};
-    c32 v = mk<float>(0.f, 0.f), vn = v;
-    if (ch.count > 0) {
-        en = ent[ch.start];
-        v = load_val(en);
-    }
-    if (ch.count > 1) nx = ent[ch.start + 1];
-    for (int e = 0; e < ch.count; ++e) {
-        BandEntry nn{};
-        if (e + 2 < ch.count) nn = ent[ch.start + e + 2];
-        if (e + 1 < ch.count) vn = load_val(nx);
-        const int dx0 = (int)(short)(en.dxy & 0xffff), dy0 = en.dxy >> 16;
-        // lane l < 8: column weight of tap l; 8 <= l < 16: row weight of tap l - 8
-        const float zf = ((float)(lane & 7) - (lane < 8 ? en.fx : en.fy)) * inv_half;
-        const float f = wlane ? es_weight_fast(zf, beta) : 0.f;
-        float wx[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) wx[c] = __shfl_sync(0xffffffffu, f, c);
-        const int ty = r - dy0;
-        const float wyr = __shfl_sync(0xffffffffu, f, 8 + (ty & 7));
-        if (ty >= 0 && ty < W) {
-            switch (dx0) {
-#define TC_BAND_CASE(D) \
-    case D: band_row_add<W, D>(acc, wx, wyr, v); break;
-                TC_BAND_CASE(-7) TC_BAND_CASE(-6) TC_BAND_CASE(-5) TC_BAND_CASE(-4)
-                TC_BAND_CASE(-3) TC_BAND_CASE(-2) TC_BAND_CASE(-1) TC_BAND_CASE(0)
-                TC_BAND_CASE(1) TC_BAND_CASE(2) TC_BAND_CASE(3) TC_BAND_CASE(4)
-                TC_BAND_CASE(5) TC_BAND_CASE(6) TC_BAND_CASE(7) TC_BAND_CASE(8)
-                TC_BAND_CASE(9) TC_BAND_CASE(10) TC_BAND_CASE(11) TC_BAND_CASE(12)
-                TC_BAND_CASE(13) TC_BAND_CASE(14) TC_BAND_CASE(15) TC_BAND_CASE(16)
-                TC_BAND_CASE(17) TC_BAND_CASE(18) TC_BAND_CASE(19) TC_BAND_CASE(20)
-                TC_BAND_CASE(21) TC_BAND_CASE(22) TC_BAND_CASE(23) TC_BAND_CASE(24)
-                TC_BAND_CASE(25) TC_BAND_CASE(26) TC_BAND_CASE(27) TC_BAND_CASE(28)
-                TC_BAND_CASE(29) TC_BAND_CASE(30) TC_BAND_CASE(31)
-#undef TC_BAND_CASE
-                default: break;
+                    for (int r = 0; r < RP / 2; r += 2) {
+                        const float4 a = cells(r, l), z = cells(r + 1, l);
+                        float4 o = odd ? a : z;
+                        o.x = __shfl_xor_sync(0xffffffffu, o.x, 1);
+                        o.y = __shfl_xor_sync(0xffffffffu, o.y, 1);
+                        o.z = __shfl_xor_sync(0xffffffffu, o.z, 1);
+                        o.w = __shfl_xor_sync(0xffffffffu, o.w, 1);
+                        float4 *own = reinterpret_cast<float4 *>(col) + r + (odd ? 1 : 0);
+                        float4 *other = reinterpret_cast<float4 *>(odd ? col - nf : col + nf) + r + (odd ? 1 : 0);
+                        put(odd ? other : own, odd ? o : a, l);
+                        put(odd ? own : other, odd ? z : o, l);
+                    }
+                }
             }
+            clear();
         }
-        en = nx;
-        nx = nn;
-        v = vn;
+        cur = nx;
+        ecur = enx;
+        nx = fu;
+        enx = efu;
     }
-    // store the band: row r of slice b, column by column (the four rows of a
-    // column are 32 contiguous bytes of the column-major grid)
-    const int nbx = nf / BAND_W;
-    const int bx = ch.band % nbx, by = ch.band / nbx;
-    c32 *dst = grid + ((size_t)b * nf + bx * BAND_W) * nf + by * BAND_H + r;
-#pragma unroll
-    for (int k = 0; k < BAND_W; ++k) {
-        if (ch.shared) {
-            atomicAdd(&dst[(size_t)k * nf].x, acc[k].x);
-            atomicAdd(&dst[(size_t)k * nf].y, acc[k].y);
-        } else {
-            dst[(size_t)k * nf] = mk<float>(acc[k].x, acc[k].y);
-        }
-    }
+    cp_async_wait_all();
 }
 
 // zero the bands that several chunks add into (column-major grid)
 __global__ void k_zero_bands(c32 *__restrict__ grid, const int *__restrict__ bands, int nf,
                              int nb) {
-    const int band = bands[blockIdx.x], nbx = nf / BAND_W;
-    const int bx = band % nbx, by = band / nbx;
+    const int band = bands[blockIdx.x], nby = nf / BAND_H;
+    const int by = band % nby, bx = band / nby;
     for (int q = threadIdx.x; q < nb * BAND_W * BAND_H; q += blockDim.x) {
         const int b = q / (BAND_W * BAND_H), cell = q - b * BAND_W * BAND_H;
         const int cc = cell / BAND_H, r = cell - cc * BAND_H;
@@ -913,7 +977,7 @@ __global__ void k_interp_lists(PolarDev g, int nf, int w, int ts, int ntiles,
 __global__ void k_band_lists(PolarDev g, int nf, int w, int *__restrict__ counts,
                              int *__restrict__ cursor, BandEntry *__restrict__ out,
                              unsigned stride, int nvirt) {
-    const int npts = g.P * g.D + nvirt, nbx = nf / BAND_W;
+    const int npts = g.P * g.D + nvirt, nby = nf / BAND_H;
     for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < npts; it += gridDim.x * blockDim.x) {
         const int idx = (int)(((unsigned long long)it * stride) % (unsigned)npts);
         int p, j;
@@ -933,7 +997,7 @@ __global__ void k_band_lists(PolarDev g, int nf, int w, int *__restrict__ counts
         }
         for (int a = 0; a < ny; ++a)
             for (int b = 0; b < nx; ++b) {
-                const int band = bys[a] * nbx + bxs[b];
+                const int band = bxs[b] * nby + bys[a];
                 if (!cursor) {
                     atomicAdd(counts + band, 1);
                     continue;
@@ -959,7 +1023,7 @@ int SpreadBands::build(const PolarDev &g, int nf_, int w_, int chunk_, int nvirt
     w = w_;
     chunk = chunk_;
     nvirt = nvirt_;
-    const int nbx = nf / BAND_W, nbands = nbx * (nf / BAND_H);
+    const int nbands = (nf / BAND_W) * (nf / BAND_H);
     const int npts = g.P * g.D + nvirt;
     DevBuf d_counts, d_cursor;
     TC_TRY(d_counts.reserve((size_t)nbands * sizeof(int)));
@@ -982,15 +1046,21 @@ int SpreadBands::build(const PolarDev &g, int nf_, int w_, int chunk_, int nvirt
                                     1u, nvirt);
         TC_LAUNCH_CHECK();
     }
+    // small problems take shorter chunks, so that every warp of the GPU gets
+    // some of the dense bands at the centre (256^2, 180 angles: 64 entries
+    // 34 us per back-projection, 256 entries 38 us)
+    const long long share = (long long)total / (148 * 24 * 2);
+    const int limit = (int)std::min<long long>(chunk, std::max<long long>(64, share));
     std::vector<BandChunk> cv;
     std::vector<int> sv;
+    cv.reserve((size_t)nbands + total / limit + 1);
     for (int b = 0; b < nbands; ++b) {
         const int c = counts[b];
-        const int n = std::max(1, ceil_div(c, chunk));
+        const int n = std::max(1, ceil_div(c, limit));
         if (n > 1) sv.push_back(b);
         for (int k = 0; k < n; ++k)
-            cv.push_back(BandChunk{b, start[b] + k * chunk,
-                                   std::max(0, std::min(chunk, c - k * chunk)), n > 1 ? 1 : 0});
+            cv.push_back(BandChunk{b, start[b] + k * limit,
+                                   std::max(0, std::min(limit, c - k * limit)), n > 1 ? 1 : 0});
     }
     nchunk = (int)cv.size();
     nshared = (int)sv.size();
@@ -1173,43 +1243,37 @@ static int spread_band_pass(const c32 *cpts, const SpreadBands &sb, const PolarD
         k_zero_bands<<<sb.nshared, 256, 0, st>>>(grid, sb.shared_bands.as<int>(), sb.nf, nb);
         TC_LAUNCH_CHECK();
     }
-    auto launch = [&](auto kern) -> int {
-        const size_t smem = (size_t)BAND_WARPS * nb * BAND_H * BAND_RS * sizeof(c32);
+    if (nb < 1 || nb > BAND_LINES) TC_FAIL(TC_ERR_ARG, "chunk too large");
+    int dev = 0, nsm = 0;
+    TC_CUDA(cudaGetDevice(&dev));
+    TC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    auto launch = [&](auto kern, int ctas) -> int {
+        const size_t smem = BAND_WARPS * sizeof(BandWarp);
         TC_TRY(set_smem(kern, smem));
-        kern<<<ceil_div(sb.nchunk, BAND_WARPS), BAND_WARPS * 32, smem, st>>>(
+        const int nblk = std::min(ceil_div(sb.nchunk, BAND_WARPS), ctas * nsm);
+        kern<<<nblk, BAND_WARPS * 32, smem, st>>>(
             cpts, grid, sb.entries.as<BandEntry>(), sb.chunks.as<BandChunk>(), sb.nchunk, sb.nf,
-            geo.P * geo.D + sb.nvirt, sb.w, beta);
+            geo.P * geo.D + sb.nvirt, beta, nb);
         TC_LAUNCH_CHECK();
         return TC_OK;
     };
-    if (nb == BAND8_NB && sb.w >= 2 && sb.w <= 8) {
-        auto launch8 = [&](auto kern) -> int {
-            kern<<<ceil_div(sb.nchunk, BAND_WARPS), BAND_WARPS * 32, 0, st>>>(
-                cpts, grid, sb.entries.as<BandEntry>(), sb.chunks.as<BandChunk>(), sb.nchunk,
-                sb.nf, geo.P * geo.D + sb.nvirt, beta);
-            TC_LAUNCH_CHECK();
-            return TC_OK;
-        };
-        switch (sb.w) {
-            case 2: return launch8(k_spread_band8<2>);
-            case 3: return launch8(k_spread_band8<3>);
-            case 4: return launch8(k_spread_band8<4>);
-            case 5: return launch8(k_spread_band8<5>);
-            case 6: return launch8(k_spread_band8<6>);
-            case 7: return launch8(k_spread_band8<7>);
-            default: return launch8(k_spread_band8<8>);
-        }
-    }
-    switch (nb) {
-        case 1: return launch(k_spread_band<1>);
-        case 2: return launch(k_spread_band<2>);
-        case 3: return launch(k_spread_band<3>);
-        case 4: return launch(k_spread_band<4>);
-        case 5: return launch(k_spread_band<5>);
-        case 6: return launch(k_spread_band<6>);
-        case 7: return launch(k_spread_band<7>);
-        case 8: return launch(k_spread_band<8>);
-        default: TC_FAIL(TC_ERR_ARG, "chunk too large");
+    // lane shapes by the chunk's lines
+    auto by_lines = [&](auto width) -> int {
+        constexpr int W = decltype(width)::value;
+        if (nb > 4) return launch(k_spread_band<W, 2, 1>, band_ctas(2));
+        if (nb > 2) return launch(k_spread_band<W, 1, 1>, band_ctas(1));
+        if (nb == 2) return launch(k_spread_band<W, 1, 2>, band_ctas(1));
+        return launch(k_spread_band<W, 1, 4>, band_ctas(1));
+    };
+    switch (sb.w) {
+        case 2: return by_lines(std::integral_constant<int, 2>());
+        case 3: return by_lines(std::integral_constant<int, 3>());
+        case 4: return by_lines(std::integral_constant<int, 4>());
+        case 5: return by_lines(std::integral_constant<int, 5>());
+        case 6: return by_lines(std::integral_constant<int, 6>());
+        case 7: return by_lines(std::integral_constant<int, 7>());
+        case 8: return by_lines(std::integral_constant<int, 8>());
+        default: TC_FAIL(TC_ERR_ARG, "spreading bands need a kernel width of 2 .. 8");
     }
 }
 

@@ -50,26 +50,26 @@ struct SpreadLists {
 };
 
 // fine-grid spreading bands of the register-FFT type-1 path: a band is
-// BAND_H rows x BAND_W columns of the fine grid, spread by one warp into its
-// own shared-memory accumulator with one point's footprint laid across the
-// lanes (BAND_H rows x 8 columns, kernel widths w <= 8).  Each entry holds
-// the point index, its first tap relative to the band (dx0, dy0 in
-// [-(w-1), band size), packed as two int16) and the tap offsets fx, fy.
-constexpr int BAND_W = 32, BAND_H = 4, BAND_CHUNK = 256;
+// BAND_H rows x BAND_W columns of the fine grid, held in a warp's registers
+// while the points whose taps touch it are added (kernel widths w <= 8).
+// Each entry holds the point index, its first tap relative to the band (dx0,
+// dy0 in [-(w-1), band size), packed as two int16) and the tap offsets fx,
+// fy.
+constexpr int BAND_W = 8, BAND_H = 8, BAND_CHUNK = 256;
 struct BandEntry {
     int pt;
     int dxy;      // (dy0 << 16) | (dx0 & 0xffff)
     float fx, fy;
 };
 struct BandChunk {
-    int band;     // by * (nf / BAND_W) + bx
+    int band;     // bx * (nf / BAND_H) + by: neighbours share their columns
     int start;    // offset into the entries
     int count;    // entries in this chunk (<= BAND_CHUNK)
     int shared;   // 1: the band is split over several chunks
 };
 struct SpreadBands {
     int nf = 0, w = 0, nvirt = 0;
-    int chunk = BAND_CHUNK;       // points per warp chunk of a band's list
+    int chunk = BAND_CHUNK;       // most points per warp chunk of a band's list
     int nchunk = 0, nshared = 0;
     DevBuf entries;               // BandEntry
     DevBuf chunks;                // BandChunk
