@@ -63,7 +63,12 @@ Plan::~Plan() {
 // few graph nodes) rather than one L2-resident pair at a time.
 constexpr size_t TOE_CHUNK_BYTES = size_t(8) << 30;
 
-int plan_build(Plan &pl, const tc_geom &g) {
+// What a plan is built for: a caller's own plan serves every operator; the
+// host entry points' plans, which live for one call, only build the point
+// lists that call uses.
+enum PlanUse { PLAN_RADON = 1, PLAN_IRADON = 2, PLAN_ALL = 3 };
+
+static int plan_build(Plan &pl, const tc_geom &g, int use) {
     if (g.n < 4) TC_FAIL(TC_ERR_SHAPE, "n must be >= 4");
     if (g.nproj < 1) TC_FAIL(TC_ERR_SHAPE, "nproj must be >= 1");
     if (!g.angles) TC_FAIL(TC_ERR_ARG, "angles is NULL");
@@ -122,10 +127,12 @@ int plan_build(Plan &pl, const tc_geom &g) {
     TC_CUDA(cudaMemcpy(pl.d_corr.ptr, corrf.data(), pl.N * sizeof(float), cudaMemcpyHostToDevice));
 
     PhaseTrace tr;
-    TC_TRY(pl.fft_D.init(pl.N));
     TC_TRY(pl.fft_nf.init(pl.nf));
     TC_TRY(pl.fft_M.init(pl.M));
     TC_TRY(det_fast_setup(pl));
+    // the general engine's detector DFT, where the register FFT does not
+    // serve both directions
+    if (!(pl.det_M && t1_fast_supported(pl.nf))) TC_TRY(pl.fft_D.init(pl.N));
     tr.mark("plan.fft_tables");
     // chunking
     const size_t pair_bytes = pl.toe_fast ? toeplitz_fast_pair_bytes(pl.N, pl.M)
@@ -157,17 +164,23 @@ int plan_build(Plan &pl, const tc_geom &g) {
     // an explicit chunk size caps the Toeplitz chunk too (slice pairs)
     if (g.max_batch > 0) pl.toe_pairs = std::min(pl.toe_pairs, std::max(1, g.max_batch / 2));
 
-    // type-1 spreading lists: measured choice of tile and sub-problem size,
-    // or the default 32 x 32 tiles of at most 2048 points
-    if (g.flags & TC_PLAN_AUTOTUNE) TC_TRY(spread_autotune(pl, cs, sn));
-    else TC_TRY(pl.spread.build(pl.geo, cs, sn, pl.nf, pl.es.w, 2048, SPREAD_TILE));
-    // bands of the register-FFT path (kernel widths <= 8)
-    if (t1_fast_supported(pl.nf) && pl.es.w <= 8) {
+    // bands of the register-FFT path (kernel widths <= 8); else, and for the
+    // autotuner to measure, type-1 spreading tiles: the measured choice of
+    // tile and sub-problem size, or 32 x 32 tiles of at most 2048 points
+    const bool bands = t1_fast_supported(pl.nf) && pl.es.w <= 8;
+    if (g.flags & TC_PLAN_AUTOTUNE) {
+        TC_TRY(spread_autotune(pl, cs, sn));
+    } else if (!bands) {
+        TC_TRY(pl.spread.build(pl.geo, cs, sn, pl.nf, pl.es.w, 2048, SPREAD_TILE));
+    } else {
+        pl.spread.nf = pl.nf;  // no tiles: the bands spread every type-1 transform
+    }
+    if (bands && (use & PLAN_IRADON)) {
         TC_TRY(pl.bands.build(pl.geo, pl.nf, pl.es.w, BAND_CHUNK, pl.nvirt));
         if (g.flags & TC_PLAN_AUTOTUNE) TC_TRY(band_autotune(pl));
     }
     // interpolation tiles of the register-FFT type-2 path
-    if (interp_tiles_apply(pl)) {
+    if (interp_tiles_apply(pl) && (use & PLAN_RADON)) {
         if (g.flags & TC_PLAN_AUTOTUNE) TC_TRY(interp_autotune(pl));
         else TC_TRY(pl.itiles.build(pl.geo, pl.nf, pl.es.w, INTERP_TILE, INTERP_POINTS, pl.nvirt));
     }
@@ -241,16 +254,18 @@ int tc_release_cached_memory(void) {
     });
 }
 
-int tc_plan_create(const tc_geom *geom, tc_plan **out) {
+static int plan_create(const tc_geom *geom, tc_plan **out, int use) {
     return guarded([&]() -> int {
         if (!geom || !out) TC_FAIL(TC_ERR_ARG, "NULL argument to tc_plan_create");
         *out = nullptr;
         std::unique_ptr<tc_plan> p(new tc_plan());
-        TC_TRY(plan_build(p->impl, *geom));
+        TC_TRY(plan_build(p->impl, *geom, use));
         *out = p.release();
         return TC_OK;
     });
 }
+
+int tc_plan_create(const tc_geom *geom, tc_plan **out) { return plan_create(geom, out, PLAN_ALL); }
 
 int tc_plan_destroy(tc_plan *plan) {
     if (!plan) return TC_OK;
@@ -500,7 +515,7 @@ int tc_radon_host(const float *img, int nslices, int n, const float *angles, int
         if (nslices < 1) TC_FAIL(TC_ERR_SHAPE, "nslices must be >= 1");
         tc_geom g{n, nproj, angles, 0.0, 0, TC_PLAN_NO_PSF};
         tc_plan *pl = nullptr;
-        TC_TRY(tc_plan_create(&g, &pl));
+        TC_TRY(plan_create(&g, &pl, PLAN_RADON));
         std::unique_ptr<tc_plan, int (*)(tc_plan *)> guard(pl, tc_plan_destroy);
         const size_t ni = (size_t)nslices * n * n, no = (size_t)nslices * nproj * n;
         DevArr di, dout;
@@ -524,7 +539,7 @@ int tc_backproject_host(const float *sino, int nslices, int nproj, int ndet, con
         const int D2 = ndet + 2 * npad;
         tc_geom g{D2, nproj, angles, 0.0, 0, TC_PLAN_NO_PSF};
         tc_plan *pl = nullptr;
-        TC_TRY(tc_plan_create(&g, &pl));
+        TC_TRY(plan_create(&g, &pl, PLAN_IRADON));
         std::unique_ptr<tc_plan, int (*)(tc_plan *)> guard(pl, tc_plan_destroy);
         const size_t ns = (size_t)nslices * nproj * ndet, ns2 = (size_t)nslices * nproj * D2;
         const size_t nx2 = (size_t)nslices * D2 * D2, nx = (size_t)nslices * ndet * ndet;
@@ -583,7 +598,7 @@ int tc_mbir_host(const float *sino, int nslices, int nproj, int ndet, const floa
         {
             tc_geom g0{ndet, nproj, angles, 0.0, 0, TC_PLAN_NO_PSF};
             tc_plan *p0 = nullptr;
-            TC_TRY(tc_plan_create(&g0, &p0));
+            TC_TRY(plan_create(&g0, &p0, PLAN_IRADON));
             std::unique_ptr<tc_plan, int (*)(tc_plan *)> guard0(p0, tc_plan_destroy);
             tr.mark("fbp.plan");
             TC_TRY(tc_iradon(p0, ds.p<float>(), dx0.p<float>(), nslices, 1, nullptr));
@@ -606,7 +621,7 @@ int tc_mbir_host(const float *sino, int nslices, int nproj, int ndet, const floa
         tr.mark("pad");
         tc_geom g{D2, nproj, angles, 0.0, 0, 0};
         tc_plan *pl = nullptr;
-        TC_TRY(tc_plan_create(&g, &pl));
+        TC_TRY(plan_create(&g, &pl, PLAN_IRADON));
         std::unique_ptr<tc_plan, int (*)(tc_plan *)> guard(pl, tc_plan_destroy);
         tr.mark("plan");
         // A^T y and |y|^2 (src/mbir2.cpp:73-77)

@@ -159,7 +159,6 @@ struct Plan {
 };
 
 // ---- operator launchers (all on `st`, device pointers) -------------------
-int plan_build(Plan &pl, const tc_geom &g);
 int psf_finish(Plan &pl);  // spectrum + Lipschitz constant from d_psf
 int radon_chunk(Plan &pl, const float *x, float *sino, int nb, cudaStream_t st);
 int iradon_chunk(Plan &pl, const float *sino, float *x, int nb, int ramp, cudaStream_t st);
