@@ -452,8 +452,8 @@ def main():
     iteration_roofline["frac"] = iteration_roofline["achieved"] / peak
 
     # ---- kernel launches inside the timed region -----------------------------
-    # begin, the two update forms (one returns at once), decide and 3 passes per chunk
-    gpu_launches = attempts * (4 + 3 * chunks)
+    # the two update forms (one returns at once), decide and 3 passes per chunk
+    gpu_launches = attempts * (3 + 3 * chunks)
 
     # ---- end to end through the reference binding ------------------------------
     e2e = None

@@ -4,13 +4,13 @@
 // Optimizer::run2 of src/optimize.h:96-154: its own beta/theta, step,
 // backtracking and iteration count) and its own buffers; what is shared is
 // the launch.  One attempt of all running scans is
-//   begin    one thread per scan
-//   update   one CTA per (scan, 32 x 16 tile): the fused stencil + Nesterov
+//   update   one CTA per (scan, 64 x 32 tile): the fused stencil + Nesterov
 //            update body of the single-volume solver
 //   rows     one CTA per (scan, slice pair, block of rows)   \  Toeplitz H new,
 //   cols     one CTA per (scan, slice pair, block of columns) | register FFT of
 //   out      one CTA per (scan, slice pair, block of rows)   /  the scan's size
-//   decide   one CTA per scan: reduce, step test, bookkeeping
+//   decide   one CTA per scan: reduce, step test, bookkeeping, beta and theta
+//            of the scan's next attempt
 //   cond     one thread: continue while any scan runs
 // so the launch count per attempt does not grow with the number of scans,
 // and the loop runs as one CUDA graph (WHILE node) or from the host.  A scan
@@ -248,11 +248,6 @@ __global__ void __launch_bounds__(UT, UPD_MIN_BLOCKS) k_batch_update(const BScan
         update_body<false>(d.X, d.H, d.aty, d.S, d.N, d.N, d.vol, d.pp, st, part, c0, r0);
 }
 
-__global__ void k_batch_begin(const BScan *__restrict__ scans, int nscans) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < nscans && scans[s].st->cond) mbir_begin(scans[s].st);
-}
-
 __global__ void k_batch_decide(const BScan *__restrict__ scans, const double *__restrict__ pu,
                                const double *__restrict__ pt) {
     const BScan &d = scans[blockIdx.x];
@@ -264,7 +259,7 @@ __global__ void k_batch_decide(const BScan *__restrict__ scans, const double *__
         for (int k = 0; k < NU; ++k) u[k] += a[(size_t)i * NU + k];
     for (int i = threadIdx.x; i < d.nt; i += blockDim.x) u[NU] += pt[d.pt_base + i];
     block_sum<NU + 1>(u);
-    if (threadIdx.x == 0) mbir_decide_core(d.st, u, d.hist);
+    if (threadIdx.x == 0 && mbir_decide_core(d.st, u, d.hist)) mbir_begin(d.st);
 }
 
 __global__ void k_batch_cond(const BScan *__restrict__ scans, int nscans, int *any,
@@ -291,8 +286,6 @@ struct BatchRun {
 
 static int enqueue_batch(const BatchRun &b, cudaStream_t s, cudaGraphConditionalHandle h,
                          int use_graph) {
-    k_batch_begin<<<ceil_div(b.nscans, 128), 128, 0, s>>>(b.scans, b.nscans);
-    TC_LAUNCH_CHECK();
     k_batch_update<<<b.nupd, UT, UPD_SMEM, s>>>(b.scans, b.upd, b.pu);
     TC_LAUNCH_CHECK();
     k_batch_rows<<<b.nrows, BT, BT_SMEM, s>>>(b.scans, b.rows);
@@ -413,6 +406,7 @@ int mbir_batched(const std::vector<BatchScanIn> &in, int num_iters, int use_grap
         h.num_iters = K;
         h.max_attempts = max_attempts > 0 ? max_attempts : 1000;
         h.cond = K > 0 ? 1 : 0;
+        mbir_begin(&h);
         TC_CUDA(cudaMemcpyAsync(b.X, in[i].x, b.vol * sizeof(float), cudaMemcpyDeviceToDevice, st));
         // H x0 on the scan's own plan (set-up; per scan)
         const int chunk = 2 * pl.toe_pairs;

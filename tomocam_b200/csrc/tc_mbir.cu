@@ -2,8 +2,7 @@
 // src/optimize.h:96-154, with the gradient and objective of
 // src/mbir2.cpp:122-136).
 //
-// One backtracking attempt is four launches:
-//   begin   beta = tnew (1/t - 1), tnew = theta(t)              (1 thread)
+// One backtracking attempt is the update, the Toeplitz passes and a decision:
 //   update  y = sol + beta (sol - x), Hy = (1+beta) H sol - beta H x,
 //           g = Hy - A^T y + w * qGGMRF'(y), new = y - step g, partial sums
 //           of y.Hy, y.A^Ty, g.g, new.A^Ty, |new - x|^2 (FP32 over 8 slices
@@ -11,7 +10,8 @@
 //           specialised for x == sol, the attempt after an accepted step)
 //   H new   Toeplitz passes, FP64 partials of new.H new
 //   decide  sqrt f(new) > sqrt f(y) + step/2 |g|^2 ? shrink step, retry from
-//           new : accept (x = sol = new), record, count      (1 CTA)
+//           new : accept (x = sol = new), record, count; then beta and theta
+//           of the next attempt                               (1 CTA)
 // H is linear, so H y never needs its own transform: every attempt costs one
 // Toeplitz application.  The iterate, H-image and scalar state live on the
 // device; three rotating buffers hold x, sol and the new iterate, and the
@@ -28,23 +28,45 @@
 
 namespace tc {
 
-__global__ void k_mbir_begin(MbirState *s) { mbir_begin(s); }
-
 // Both forms are launched every attempt and the one that does not apply
 // returns at once (x == sol after an accepted step, x != sol after a
 // rejected one), so each gets its own register allocation.
 // tmap (use_tma != 0): the three iterate buffers as one [3 S][R][C] float
 // tensor with a 72 x 34 x 1 box, for the x == sol form's plane tiles.
+// blockIdx.z: planes blockIdx.z * zc .. + zc - 1 of the volume.
 template <bool SAME>
 __global__ void __launch_bounds__(UT, UPD_MIN_BLOCKS)
 k_mbir_update(float *__restrict__ X, const float *__restrict__ H, const float *__restrict__ aty,
               int S, int R, int C, size_t vol, PriorParams pp, const MbirState *__restrict__ st,
-              double *__restrict__ partials, const __grid_constant__ CUtensorMap tmap, int use_tma) {
+              double *__restrict__ partials, const __grid_constant__ CUtensorMap tmap, int use_tma,
+              int zc) {
     if ((st->ix == st->isol) != SAME) return;
-    double *part = partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * NU;
-    const int c0 = blockIdx.x * UX, r0 = blockIdx.y * UY;
-    update_body<SAME>(X, H, aty, S, R, C, vol, pp, st, part, c0, r0, 0, 1 << 30,
+    double *part =
+        partials + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * NU;
+    const int c0 = blockIdx.x * UX, r0 = blockIdx.y * UY, s_lo = blockIdx.z * zc;
+    update_body<SAME>(X, H, aty, S, R, C, vol, pp, st, part, c0, r0, s_lo, s_lo + zc,
                       use_tma ? &tmap : nullptr);
+}
+
+// Planes per CTA of the update: where the tiles alone leave CTA slots idle
+// the volume is split in z, at multiples of the slices summed in FP32 (so the
+// split does not change what is summed).  A run costs its planes, one more
+// for the plane below it and about one of start-up; the split with the
+// smallest (waves of CTAs) x (planes per CTA) is taken.  Update of 24 slices
+// of 300^2 (50 tiles for 296 slots; runs of 8) 0.165 -> 0.084 ms, of 64 x
+// 128^2 0.379 -> 0.066, of 33 x 500^2 0.224 -> 0.177; 16 x 1024^2 and larger
+// volumes keep one run.
+static int update_run(int tiles, int S, int slots) {
+    int best = S;
+    double cost = (double)ceil_div(tiles, slots) * (S + 1.0);
+    for (int zc = ACC_CHUNK; zc < S; zc += ACC_CHUNK) {
+        const double c = (double)ceil_div(tiles * ceil_div(S, zc), slots) * (zc + 2.0);
+        if (c < cost) {
+            cost = c;
+            best = zc;
+        }
+    }
+    return best;
 }
 
 // The tensor map of the iterate buffers for the update's plane tiles, or
@@ -87,6 +109,7 @@ __global__ void k_mbir_decide(MbirState *s, const double *__restrict__ pu, int n
     block_sum<NU + 1>(u);
     if (threadIdx.x != 0) return;
     const int cond = mbir_decide_core(s, u, hist);
+    if (cond) mbir_begin(s);
     if (use_graph) cudaGraphSetConditional(handle, cond);
 }
 
@@ -102,6 +125,7 @@ struct MbirRun {
     MbirState *st;
     double *pu, *pt, *hist;
     int nu, nt;
+    int zc;            // planes per CTA of the update
     PriorParams pp;
     CUtensorMap tmap;  // iterate buffers, for the update's plane tiles
     int use_tma;
@@ -113,15 +137,13 @@ static int enqueue_attempt(MbirRun &m, cudaStream_t s, cudaGraphConditionalHandl
                            cudaEvent_t *ev = nullptr) {
     Plan &pl = *m.pl;
     const int N = pl.N;
-    k_mbir_begin<<<1, 1, 0, s>>>(m.st);
-    TC_LAUNCH_CHECK();
     if (ev) TC_CUDA(cudaEventRecord(ev[0], s));
-    dim3 grid(ceil_div(N, UX), ceil_div(N, UY));
+    dim3 grid(ceil_div(N, UX), ceil_div(N, UY), ceil_div(m.S, m.zc));
     k_mbir_update<true><<<grid, UT, UPD_SMEM, s>>>(m.X, m.H, m.aty, m.S, N, N, m.vol, m.pp, m.st,
-                                                   m.pu, m.tmap, m.use_tma);
+                                                   m.pu, m.tmap, m.use_tma, m.zc);
     TC_LAUNCH_CHECK();
     k_mbir_update<false><<<grid, UT, UPD_SMEM, s>>>(m.X, m.H, m.aty, m.S, N, N, m.vol, m.pp, m.st,
-                                                    m.pu, m.tmap, 0);
+                                                    m.pu, m.tmap, 0, m.zc);
     TC_LAUNCH_CHECK();
     if (ev) TC_CUDA(cudaEventRecord(ev[1], s));
     const int chunk = 2 * pl.toe_pairs;
@@ -171,7 +193,12 @@ int mbir_solve(Plan &pl, const float *aty, double sino_sq, float *x, int S,
     m.S = S;
     m.vol = vol;
     m.aty = aty;
-    m.nu = ceil_div(N, UX) * ceil_div(N, UY);
+    int dev = 0, nsm = 0;
+    TC_CUDA(cudaGetDevice(&dev));
+    TC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int tiles = ceil_div(N, UX) * ceil_div(N, UY);
+    m.zc = update_run(tiles, S, UPD_MIN_BLOCKS * nsm);
+    m.nu = tiles * ceil_div(S, m.zc);
     // two CTAs per SM need 2 x UPD_SMEM of the unified L1 / shared array;
     // state the carveout so launches from a graph get the same split
     TC_CUDA(cudaFuncSetAttribute(k_mbir_update<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM));
@@ -213,6 +240,7 @@ int mbir_solve(Plan &pl, const float *aty, double sino_sq, float *x, int S,
     h.num_iters = K;
     h.max_attempts = o.max_attempts > 0 ? o.max_attempts : 1000;
     h.cond = K > 0 ? 1 : 0;
+    mbir_begin(&h);
     TC_CUDA(cudaMemcpyAsync(m.st, &h, sizeof(h), cudaMemcpyHostToDevice, st));
     TC_CUDA(cudaMemcpyAsync(m.X, x, vol * sizeof(float), cudaMemcpyDeviceToDevice, st));
     // H x0

@@ -21,8 +21,9 @@ struct MbirState {
     int status;                // 0 ok, 1 backtracking cap reached, 3 a bounded device wait gave up
 };
 
-// beta and theta for the next attempt (src/optimize.h:117-121)
-__device__ __forceinline__ void mbir_begin(MbirState *s) {
+// beta and theta for the next attempt (src/optimize.h:117-121); the host sets
+// them for the first attempt, the decision for those after it
+__host__ __device__ __forceinline__ void mbir_begin(MbirState *s) {
     const double t = s->t;
     s->beta = s->tnew * (1.0 / t - 1.0);
     s->tnew = 0.5 * (sqrt(t * t * t * t + 4.0 * t * t) - t * t);

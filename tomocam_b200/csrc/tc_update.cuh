@@ -379,7 +379,9 @@ __device__ __forceinline__ void import_edges(UpdRegs &r, const float *es, int vb
 // ---------------------------------------------------------------------------
 // SAME: x == sol (every attempt after an accepted step), so y = sol, H y =
 // H sol and neither x nor H x is read.  Planes s_lo .. s_hi-1 are written and
-// summed; the others (the halo planes of a slab) only serve as neighbours.
+// summed; the others (the halo planes of a slab, the planes of the CTAs above
+// and below where the march is split in z) only serve as neighbours: the
+// march starts one plane below s_lo, whose dz = 1 edges plane s_lo needs.
 template <bool SAME>
 __device__ __forceinline__ void update_body(float *__restrict__ X, const float *__restrict__ H,
                                             const float *__restrict__ aty, int S, int R, int C,
@@ -539,6 +541,7 @@ __device__ __forceinline__ void update_body(float *__restrict__ X, const float *
     };
 
     // the block's voxel data (A^T y, H sol, and for !SAME H x and x) for a plane
+    const int s_beg = max(s_lo - 1, 0), s_end = min(s_hi, S);
     const int gr0 = r0 + y0, gc0 = c0 + x0;
     const bool row_in[2] = {gr0 < R, gr0 + 1 < R};
     const bool full4 = vec && gc0 + 3 < C;
@@ -554,7 +557,7 @@ __device__ __forceinline__ void update_body(float *__restrict__ X, const float *
         }
     };
     auto fetch_vox = [&](int s) {
-        if (s >= S) return;
+        if (s >= s_end) return;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if (!row_in[q] || gc0 >= C) continue;
@@ -610,7 +613,7 @@ __device__ __forceinline__ void update_body(float *__restrict__ X, const float *
 #pragma unroll
     for (int v = 0; v < BV; ++v) r.pnext[v] = 0.f;
 
-    // planes 0 and 1 resident, the voxel data of plane 0 in flight
+    // planes s_beg and s_beg + 1 resident, the voxel data of s_beg in flight
     if (tma) {
         if (tid == 0) {
 #pragma unroll
@@ -618,33 +621,35 @@ __device__ __forceinline__ void update_body(float *__restrict__ X, const float *
             mbar_fence_init();
         }
         __syncthreads();
-        tma_plane(0, 0);
-        tma_plane(1, 1);
+        tma_plane(s_beg, 0);
+        tma_plane(s_beg + 1, 1);
         tma_wait(0);
         __syncthreads();
         tma_wait(1);
     } else if (SAME) {
-        copy_plane(0, yp);
-        copy_plane(1, yp + PNA);
+        copy_plane(s_beg, yp);
+        copy_plane(s_beg + 1, yp + PNA);
         cp_async_wait_all();
     } else {
-        fetch_y(0);
+        fetch_y(s_beg);
         store_y(yp);
-        fetch_y(1);
+        fetch_y(s_beg + 1);
         store_y(yp + PNA);
     }
-    fetch_vox(0);
+    fetch_vox(s_beg);
     __syncthreads();
-    // seed: the dz = 1 edges from plane -1 (clamped to plane 0) into plane 0
     load_window(yp);
     shift_window();
-    own_edges<0, true>(r, pp, es + vb * SLOTS);
-    halo_edges(yp, yp, true);
-    __syncthreads();
-    import_edges<0, true>(r, es, vb);
+    if (s_beg == 0) {
+        // seed: the dz = 1 edges from plane -1 (clamped to plane 0) into plane 0
+        own_edges<0, true>(r, pp, es + vb * SLOTS);
+        halo_edges(yp, yp, true);
+        __syncthreads();
+        import_edges<0, true>(r, es, vb);
+    }
 
     int bc = 0;  // buffer of plane s (plane s+1 in bc+1, s+2 in bc+2, mod 3)
-    for (int s = 0; s < S; ++s) {
+    for (int s = s_beg; s < s_end; ++s) {
         const int b1 = bc == 2 ? 0 : bc + 1, b2 = b1 == 2 ? 0 : b1 + 1;
         float *ycur = yp + bc * PNA, *ynxt = yp + b1 * PNA, *yfill = yp + b2 * PNA;
         // plane s+1 resident; the last step's imports done; plane s-1 free;
@@ -684,7 +689,7 @@ __device__ __forceinline__ void update_body(float *__restrict__ X, const float *
         }
         fetch_vox(s + 1);
         import_edges<0, false>(r, es, vb);
-        if (s >= s_lo && s < s_hi) {
+        if (s >= s_lo) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 if (!row_in[q] || gc0 >= C) continue;
@@ -721,7 +726,7 @@ __device__ __forceinline__ void update_body(float *__restrict__ X, const float *
             }
         }
         shift_window();
-        if ((s % ACC_CHUNK) == ACC_CHUNK - 1 || s == S - 1) {
+        if ((s % ACC_CHUNK) == ACC_CHUNK - 1 || s == s_end - 1) {
 #pragma unroll
             for (int k = 0; k < NU; ++k) {
                 accs[k * UT + tid] += (double)cacc[k];
