@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "tc_cpasync.cuh"
 #include "tc_fft_fast.cuh"
 #include "tc_mbir.cuh"
 
@@ -51,7 +52,8 @@ constexpr int BT = 512;  // threads per CTA of the batched Toeplitz passes
 template <class F>
 struct BShape {
     static constexpr int L = BT / F::T;  // lines per CTA
-    static constexpr int STAGE = L * F::M + F::M / 16;
+    static constexpr int STAGE = L * F::M + 2 * (F::M / 16);
+    static_assert(L % 2 == 0, "the output pass copies two rows per 16-byte piece");
     static constexpr int SMEM = (L * F::LS > STAGE) ? L * F::LS : STAGE;  // complex
 };
 
@@ -68,6 +70,23 @@ constexpr int BT_SMEM_C =
     cmax(cmax(cmax(BShape<B64>::SMEM, BShape<B128>::SMEM), cmax(BShape<B256>::SMEM, BShape<B512>::SMEM)),
          cmax(cmax(BShape<B1024>::SMEM, BShape<B2048>::SMEM), BShape<B4096>::SMEM));
 constexpr int BT_SMEM = BT_SMEM_C * (int)sizeof(c32);
+
+// The column pass runs CTAs of 256 threads, BCT / (M / 16) lines: a column is
+// loaded, transformed twice and stored with no other work to hide its memory
+// latency but the other CTAs of the SM.  24 scans of 256^2 .. 1024^2, per
+// attempt: one CTA of 512 threads 365 us; two of 256 (128 registers) 284,
+// three (80 registers, some spilled) 273, four 294.
+constexpr int BCT = 256;
+constexpr int BCOLS = 3;
+template <class F>
+struct BColShape {
+    static constexpr int L = BCT / F::T;
+    static constexpr int SMEM = L * F::LS;
+};
+constexpr int BCT_SMEM =
+    (int)sizeof(c32) *
+    cmax(cmax(cmax(BColShape<B64>::SMEM, BColShape<B128>::SMEM), cmax(BColShape<B256>::SMEM, BColShape<B512>::SMEM)),
+         cmax(cmax(BColShape<B1024>::SMEM, BColShape<B2048>::SMEM), BColShape<B4096>::SMEM));
 
 template <int L>
 __device__ __forceinline__ int bstg(int pos, int l) { return pos * L + l + (pos >> 4); }
@@ -104,7 +123,7 @@ __device__ __forceinline__ void brows(const BScan &d, int q, int rb, c32 *sm) {
 
 template <class F>
 __device__ __forceinline__ void bcols(const BScan &d, int q, int pg, c32 *sm) {
-    constexpr int L = BShape<F>::L;
+    constexpr int L = BColShape<F>::L;
     const int l = threadIdx.x / F::T, t = threadIdx.x % F::T;
     // with more lines per CTA than columns (M = 64) the surplus lines only
     // take part in the barriers
@@ -147,14 +166,22 @@ __device__ __forceinline__ void bout(const BScan &d, int q, int rb, c32 *sm, dou
     const int N = d.N, r0 = rb * L, r = r0 + l;
     const bool valid = r < N, has_b = 2 * q + 1 < d.S;
     const c32 *Wq = d.W + (size_t)q * F::M * d.NS + r0;
-    for (int e = threadIdx.x; e < F::M * L; e += BT) {
-        const int pos = e / L, ll = e % L;
-        sm[bstg<L>(pos, ll)] = (r0 + ll < N) ? Wq[(size_t)pos * d.NS + ll] : mk<float>(0.f, 0.f);
+    // two rows per 16-byte piece, all pieces in flight (250 us per attempt of
+    // the 24 scans with loads through registers, 163 so); a piece whose first
+    // row is an image row may carry a second one past them (in the stride's
+    // padding), whose line is transformed and dropped
+    auto slot = [](int pos, int ll) { return pos * L + ll + 2 * (pos >> 4); };
+    for (int e = threadIdx.x; e < F::M * L / 2; e += BT) {
+        const int pos = e / (L / 2), ll = 2 * (e % (L / 2));
+        if (r0 + ll < N) cp_async16(sm + slot(pos, ll), Wq + (size_t)pos * d.NS + ll);
+        else sm[slot(pos, ll)] = sm[slot(pos, ll + 1)] = mk<float>(0.f, 0.f);
     }
+    cp_async_commit();
+    cp_async_wait_all();
     __syncthreads();
     c32 v[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = sm[bstg<L>(t * 16 + i, l)];
+    for (int i = 0; i < 16; ++i) v[i] = sm[slot(t * 16 + i, l)];
     __syncthreads();
     F::inverse(v, sm + l * F::LS, t, d.tw);
     const size_t off = (size_t)d.st->inew * d.vol;
@@ -205,7 +232,7 @@ __global__ void __launch_bounds__(BT, 2) k_batch_rows(const BScan *__restrict__ 
 #undef CALL_ROWS
 }
 
-__global__ void __launch_bounds__(BT, 1) k_batch_cols(const BScan *__restrict__ scans,
+__global__ void __launch_bounds__(BCT, BCOLS) k_batch_cols(const BScan *__restrict__ scans,
                                                      const int4 *__restrict__ items) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     c32 *sm = reinterpret_cast<c32 *>(smem_raw);
@@ -290,7 +317,7 @@ static int enqueue_batch(const BatchRun &b, cudaStream_t s, cudaGraphConditional
     TC_LAUNCH_CHECK();
     k_batch_rows<<<b.nrows, BT, BT_SMEM, s>>>(b.scans, b.rows);
     TC_LAUNCH_CHECK();
-    k_batch_cols<<<b.ncols, BT, BT_SMEM, s>>>(b.scans, b.cols);
+    k_batch_cols<<<b.ncols, BCT, BCT_SMEM, s>>>(b.scans, b.cols);
     TC_LAUNCH_CHECK();
     k_batch_out<<<b.nout, BT, BT_SMEM, s>>>(b.scans, b.out, b.pt);
     TC_LAUNCH_CHECK();
@@ -302,6 +329,7 @@ static int enqueue_batch(const BatchRun &b, cudaStream_t s, cudaGraphConditional
 }
 
 static int lines_per_cta(int M) { return BT / (M / 16); }
+static int cols_per_cta(int M) { return BCT / (M / 16); }
 
 int mbir_batched(const std::vector<BatchScanIn> &in, int num_iters, int use_graph,
                  int max_attempts, double *history, cudaStream_t st) {
@@ -360,7 +388,7 @@ int mbir_batched(const std::vector<BatchScanIn> &in, int num_iters, int use_grap
                 rows.push_back(make_int4(i, q, rb, 0));
                 outs.push_back(make_int4(i, q, rb, 0));
             }
-            for (int pg = 0; pg < ceil_div(b.M, L); ++pg) cols.push_back(make_int4(i, q, pg, 0));
+            for (int pg = 0; pg < ceil_div(b.M, cols_per_cta(b.M)); ++pg) cols.push_back(make_int4(i, q, pg, 0));
         }
     }
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -443,7 +471,8 @@ int mbir_batched(const std::vector<BatchScanIn> &in, int num_iters, int use_grap
 
     for (const void *k : {(const void *)k_batch_rows, (const void *)k_batch_cols,
                           (const void *)k_batch_out}) {
-        TC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM));
+        TC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     k == (const void *)k_batch_cols ? BCT_SMEM : BT_SMEM));
         TC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                      cudaSharedmemCarveoutMaxShared));
     }
