@@ -70,8 +70,26 @@ __device__ __forceinline__ int mode_of(int n, int N) {
     return (r >= 0 && r < N) ? r : -1;
 }
 
+// CTAs of nt threads that make up `warps` warps on an SM.  The passes wait on
+// shared memory and barriers between stages, and more warps per SM hide that
+// until the register cap makes the transforms spill.  Measured with 16, 20,
+// 24 and 32 warps (16 slices; the lengths 512 .. 6144), each kernel takes
+// what was fastest:
+//   detector DFT   32: 1536-point 159 -> 145 us, 2048 83 -> 73, Bluestein on
+//                  2048 52 -> 45, on 1536 81 -> 66
+//   type-1 rows    24 from 1024 points on: 3072 264 -> 219 us, 2048 51 -> 35,
+//                  1024 27 -> 19 (512: 5.5 -> 6.0, so one CTA there)
+//   type-2 columns 32 at 192 threads (3072 363 -> 320 us, 1536 96 -> 86),
+//                  else 24 (4096 474 -> 445, 2048 50 -> 46; 32 there costs)
+//   type-1 columns 20 at 192 threads (3072 310 -> 294, 1536 94 -> 92), else
+//                  16 (24 cost 3 to 5 % at 1024 and 4096)
+// and two CTAs of the 384-thread lines (6144) throughout: one takes 20 to 35 %
+// longer.
+constexpr int sm_ctas(int nt, int warps) {
+    return nt == 384 ? 2 : (warps * 32 / nt < 1 ? 1 : warps * 32 / nt);
+}
 template <class F, int LC>
-__global__ void __launch_bounds__(F::T * LC, (F::T * LC <= 384) ? 2 : 1)
+__global__ void __launch_bounds__(F::T * LC, sm_ctas(F::T * LC, F::T * LC == 192 ? 20 : 16))
 k_t1f_cols(const c32 *__restrict__ G, c32 *__restrict__ Rw, int N, int NS, int nb,
            const c32 *__restrict__ tw) {
     using S = T1Shape<F>;
@@ -122,7 +140,7 @@ k_t1f_cols(const c32 *__restrict__ G, c32 *__restrict__ Rw, int N, int NS, int n
 }
 
 template <class F, int RB>
-__global__ void __launch_bounds__(F::T * RB, 1)
+__global__ void __launch_bounds__(F::T * RB, F::M >= 1024 ? sm_ctas(F::T * RB, 24) : 1)
 k_t1f_rows(const c32 *__restrict__ Rw, float *__restrict__ out, const float *__restrict__ sub,
            const float *__restrict__ corr, float scale, int N, int NS, int nb,
            const c32 *__restrict__ tw, int nslices, int pair) {
@@ -216,7 +234,7 @@ struct DetShape {
 // radon at 2908² with 1969 angles went 0.321 -> 0.297 ms per slice).
 template <class F, bool BLUE, bool INV>
 __global__ void __launch_bounds__(F::T * DetShape<F, BLUE>::LC,
-                                  (F::T * DetShape<F, BLUE>::LC <= 384) ? 2 : 1)
+                                  sm_ctas(F::T * DetShape<F, BLUE>::LC, 32))
 k_det_fast(const void *__restrict__ in, void *__restrict__ out, int D, int nlines, int ramp,
            float scale, const c32 *__restrict__ chirp, const c32 *__restrict__ bhat,
            const c32 *__restrict__ tw, int P, int nslices, int pair, size_t cstride, int nvirt) {
@@ -448,7 +466,7 @@ k_t2f_rows(const float *__restrict__ x, c32 *__restrict__ Q, const float *__rest
 }
 
 template <class F, int LC>
-__global__ void __launch_bounds__(F::T * LC, (F::T * LC <= 384) ? 2 : 1)
+__global__ void __launch_bounds__(F::T * LC, sm_ctas(F::T * LC, F::T * LC == 192 ? 32 : 24))
 k_t2f_cols(const c32 *__restrict__ Q, c32 *__restrict__ G, int N, int NS, int nb,
            const c32 *__restrict__ tw) {
     using S = T2Shape<F>;
