@@ -114,7 +114,7 @@ int qggmrf_launch(const float *x, float *g, int S, int R, int C, float sigma, fl
     int dev = 0, nsm = 0;
     TC_CUDA(cudaGetDevice(&dev));
     TC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    TC_CUDA(cudaFuncSetAttribute(k_qggmrf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(QSmem)));
+    static_assert(sizeof(QSmem) <= 48 * 1024, "no opt-in for more shared memory needed");
     const int gx = ceil_div(C, EX), gy = ceil_div(R, QTY);
     const int zc = edge_run(gx * gy, S, QCTAS * nsm);
     const dim3 grid(gx, gy, ceil_div(S, zc));

@@ -133,7 +133,7 @@ k_tpf_rows(const float *__restrict__ x, c32 *__restrict__ W, int N, int NS, int 
 // ib + s * LC + l.  The next step's lines are copied into the prefetch buffer
 // (cp.async, 16 bytes per request) while the current step is transformed.
 template <class F, int LC>
-__global__ void __launch_bounds__(F::T * LC, (F::T * LC <= 384) ? 2 : 1)
+__global__ void __launch_bounds__(F::T * LC, (F::M == 3072) ? 3 : (F::T * LC <= 384) ? 2 : 1)
 k_tpf_cols(c32 *__restrict__ W, const float *__restrict__ phatp, int N, int NS, int npairs,
            const c32 *__restrict__ tw) {
     // TIGHT: 384-thread lines (M = 6144) under the 80-register cap of two
@@ -142,8 +142,11 @@ k_tpf_cols(c32 *__restrict__ W, const float *__restrict__ phatp, int N, int NS, 
     // position, and the inverse forms the low half directly: fewer spills,
     // operator at 2908² 0.2518 -> 0.2462 ms per slice.  With more registers
     // (M = 4096: 128, no spill) holding the column is faster (0.0802
-    // against 0.0824 ms per slice).
-    constexpr bool TIGHT = F::T * LC == 384;
+    // against 0.0824 ms per slice).  M = 3072 takes three CTAs of 192 threads
+    // the same way (112 registers each): operator on 16 x 1400² 0.832 ->
+    // 0.798 ms; at M = 768 x 2^k lines per CTA and the powers of two a third
+    // CTA cost 0 to 6 %.
+    constexpr bool TIGHT = F::T * LC == 384 || F::M == 3072;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     c32 *scr = reinterpret_cast<c32 *>(smem_raw);
     c32 *pf = scr + FastShape<F>::SCR_COLS;  // [LC][NS]
