@@ -1071,21 +1071,16 @@ int SpreadBands::build(const PolarDev &g, int nf_, int w_, int chunk_, int nvirt
                                     1u, nvirt);
         TC_LAUNCH_CHECK();
     }
-    // small problems take shorter chunks, so that every warp of the GPU gets
-    // some of the dense bands at the centre (256^2, 180 angles: 64 entries
-    // 34 us per back-projection, 256 entries 38 us)
-    const long long share = (long long)total / (148 * 24 * 2);
-    const int limit = (int)std::min<long long>(chunk, std::max<long long>(64, share));
     std::vector<BandChunk> cv;
     std::vector<int> sv;
-    cv.reserve((size_t)nbands + total / limit + 1);
+    cv.reserve((size_t)nbands + total / chunk + 1);
     for (int b = 0; b < nbands; ++b) {
         const int c = counts[b];
-        const int n = std::max(1, ceil_div(c, limit));
+        const int n = std::max(1, ceil_div(c, chunk));
         if (n > 1) sv.push_back(b);
         for (int k = 0; k < n; ++k)
-            cv.push_back(BandChunk{b, start[b] + k * limit,
-                                   std::max(0, std::min(limit, c - k * limit)), n > 1 ? 1 : 0});
+            cv.push_back(BandChunk{b, start[b] + k * chunk,
+                                   std::max(0, std::min(chunk, c - k * chunk)), n > 1 ? 1 : 0});
     }
     nchunk = (int)cv.size();
     nshared = (int)sv.size();

@@ -11,9 +11,8 @@ namespace tc {
 // its 356 us on 32 slices of 768^2); with shared edges and the ring's 11 %
 // more there are 43, and it takes 272 us (16 x 2048^2: 1246 -> 918).  Now the
 // evaluations' latency bounds it (short-scoreboard and fixed-latency stalls,
-// SFU 62 % busy), and warps per SM count: six CTAs of 40 registers 272 us,
-// five 280, seven (spilling to 32 registers' worth of reloads) 293; 32 x 16
-// tiles at three CTAs 362.
+// SFU 64 % busy by its count), and warps per SM count: six CTAs of 40 registers 272 us,
+// five 280, seven (32 registers) 293; 32 x 16 tiles at three CTAs 362.
 constexpr int QTY = 8, QCTAS = 6;
 struct QSmem {
     float plane[3][EdgeTile<QTY>::PN];

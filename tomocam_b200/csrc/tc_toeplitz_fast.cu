@@ -143,9 +143,8 @@ k_tpf_cols(c32 *__restrict__ W, const float *__restrict__ phatp, int N, int NS, 
     // operator at 2908² 0.2518 -> 0.2462 ms per slice.  With more registers
     // (M = 4096: 128, no spill) holding the column is faster (0.0802
     // against 0.0824 ms per slice).  M = 3072 takes three CTAs of 192 threads
-    // the same way (112 registers each): operator on 16 x 1400² 0.832 ->
-    // 0.798 ms; at M = 768 x 2^k lines per CTA and the powers of two a third
-    // CTA cost 0 to 6 %.
+    // the same way (96 registers): operator on 16 x 1400² 0.836 -> 0.801 ms;
+    // at the other lengths a third CTA made it 0 to 6 % slower.
     constexpr bool TIGHT = F::T * LC == 384 || F::M == 3072;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     c32 *scr = reinterpret_cast<c32 *>(smem_raw);
