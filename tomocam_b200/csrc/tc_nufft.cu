@@ -25,7 +25,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <type_traits>
 
@@ -896,21 +895,30 @@ std::vector<double> es_correction(int nm, int nf, const EsKernel &es) {
             if (hm + m < nm) corr[hm + m] = c;
         }
     };
-    // a thread for every 30000 terms (about 0.4 ms), at most 8
+    // a thread for every 30000 terms (about 0.4 ms), at most 8.  Where a thread
+    // cannot be had (no thread, no memory for its state) the rest runs here;
+    // every started thread is joined before corr is handed on, on all paths
     const int nt = std::max(1, std::min(8, (int)((size_t)(hm + 1) * xq.size() / 30000)));
-    std::vector<std::thread> pool;
-    int done = 0;
-    for (int t = 0; t + 1 < nt; ++t) {
-        const int k1 = (int)((long long)(hm + 1) * (t + 1) / nt);
-        try {
-            pool.emplace_back(modes, done, k1);
-        } catch (const std::system_error &) {
-            break;  // no more threads to be had: the rest runs here
+    {
+        struct Pool {
+            std::vector<std::thread> th;
+            ~Pool() {
+                for (auto &t : th) t.join();
+            }
+        } pool;
+        pool.th.reserve(nt);
+        int done = 0;
+        for (int t = 0; t + 1 < nt; ++t) {
+            const int k1 = (int)((long long)(hm + 1) * (t + 1) / nt);
+            try {
+                pool.th.emplace_back(modes, done, k1);
+            } catch (const std::exception &) {
+                break;
+            }
+            done = k1;
         }
-        done = k1;
+        modes(done, hm + 1);
     }
-    modes(done, hm + 1);
-    for (auto &t : pool) t.join();
     return corr;
 }
 
