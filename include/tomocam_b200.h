@@ -66,8 +66,8 @@ typedef struct {
 #define TC_PLAN_NO_PSF 1
 /* tc_geom.flags: time the NUFFT's spreading and interpolation on this
  * geometry and keep the fastest choices (cached per geometry for the
- * process): tile edges (16, 32, 64) and sub-problem sizes of the type-1 tile
- * path, and on the register-FFT path the band lists' chunk (128 .. 1024
+ * process): tile edges (16, 32, 64) and sub-problem sizes where type 1 spreads
+ * on tiles, and on the register-FFT path the band lists' chunk (128 .. 1024
  * points), the slices per NUFFT chunk and the type-2 interpolation tiles
  * (edge 16 or 32, 256 .. 4096 points per sub-problem); without it 32 x 32
  * spreading tiles of at most 2048 points, 256-point band chunks, up to 8
@@ -100,7 +100,9 @@ typedef struct {
     double lipschitz;    /* max(H 1) as in src/mbir2.cpp:100-112 */
     int32_t toeplitz_pairs; /* slice pairs per Toeplitz launch */
     int32_t toeplitz_fast;  /* 1: register-resident FFT kernels */
-    int32_t spread_tile;    /* type-1 spreading tile edge */
+    int32_t spread_tile;    /* type-1 spreading tile edge; with bands (band_chunk > 0)
+                             * no tile lists are built and this and the next are
+                             * the tile path's defaults */
     int32_t spread_max_points; /* points per spreading sub-problem */
     int32_t band_chunk;     /* points per warp chunk of the band spreading (0: no bands) */
     int32_t interp_tile;    /* type-2 interpolation tile edge (0: one thread per point) */

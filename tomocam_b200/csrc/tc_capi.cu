@@ -164,20 +164,18 @@ static int plan_build(Plan &pl, const tc_geom &g, int use) {
     // an explicit chunk size caps the Toeplitz chunk too (slice pairs)
     if (g.max_batch > 0) pl.toe_pairs = std::min(pl.toe_pairs, std::max(1, g.max_batch / 2));
 
-    // bands of the register-FFT path (kernel widths <= 8); else, and for the
-    // autotuner to measure, type-1 spreading tiles: the measured choice of
-    // tile and sub-problem size, or 32 x 32 tiles of at most 2048 points
-    const bool bands = t1_fast_supported(pl.nf) && pl.es.w <= 8;
-    if (g.flags & TC_PLAN_AUTOTUNE) {
+    // type-1 spreading lists: bands on the register-FFT path (kernel widths
+    // <= 8), which then spread every type-1 transform; else tiles, 32 x 32 of
+    // at most 2048 points or the autotuner's choice
+    if (t1_fast_supported(pl.nf) && pl.es.w <= 8) {
+        if (use & PLAN_IRADON) {
+            TC_TRY(pl.bands.build(pl.geo, pl.nf, pl.es.w, BAND_CHUNK, pl.nvirt));
+            if (g.flags & TC_PLAN_AUTOTUNE) TC_TRY(band_autotune(pl));
+        }
+    } else if (g.flags & TC_PLAN_AUTOTUNE) {
         TC_TRY(spread_autotune(pl, cs, sn));
-    } else if (!bands) {
-        TC_TRY(pl.spread.build(pl.geo, cs, sn, pl.nf, pl.es.w, 2048, SPREAD_TILE));
     } else {
-        pl.spread.nf = pl.nf;  // no tiles: the bands spread every type-1 transform
-    }
-    if (bands && (use & PLAN_IRADON)) {
-        TC_TRY(pl.bands.build(pl.geo, pl.nf, pl.es.w, BAND_CHUNK, pl.nvirt));
-        if (g.flags & TC_PLAN_AUTOTUNE) TC_TRY(band_autotune(pl));
+        TC_TRY(pl.spread.build(pl.geo, cs, sn, pl.nf, pl.es.w, 2048, SPREAD_TILE));
     }
     // interpolation tiles of the register-FFT type-2 path
     if (interp_tiles_apply(pl) && (use & PLAN_RADON)) {

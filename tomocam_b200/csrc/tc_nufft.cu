@@ -1004,7 +1004,7 @@ __global__ void k_interp_lists(PolarDev g, int nf, int w, int ts, int ntiles,
 }
 
 // count (cursor == null) or place (cursor != null) every point in the lists
-// of the bands its taps touch (at most 2 band columns and 3 band rows for
+// of the bands its taps touch (at most 2 band columns and 2 band rows for
 // w <= 8), with its first tap relative to each band; the tap origin is
 // point_taps', the one the entry then carries to the spreading
 __global__ void k_band_lists(PolarDev g, int nf, int w, int *__restrict__ counts,
@@ -1313,7 +1313,10 @@ static int t1_from_points(const cpx<R> *cpts, const PolarDev &geo, const SpreadL
                           const float *sub, R scale, cudaStream_t st,
                           const SpreadBands *bands = nullptr) {
     const int nf = T.dev.L;
-    if (sl.nf != nf) TC_FAIL(TC_ERR_STATE, "spread lists built for another grid");
+    auto lists_match = [&]() -> int {
+        if (sl.nf != nf) TC_FAIL(TC_ERR_STATE, "spread lists built for another grid");
+        return TC_OK;
+    };
     if constexpr (std::is_same<R, float>::value && std::is_same<Tout, float>::value) {
         if (t1_fast_supported(nf) && !T.dev.bluestein) {
             // column-major grid, then the register-FFT passes
@@ -1321,6 +1324,7 @@ static int t1_from_points(const cpx<R> *cpts, const PolarDev &geo, const SpreadL
                 TC_TRY(spread_band_pass(cpts, *bands, geo, (float)es.beta, nb, grid, st));
                 return t1_fast_fft(grid, rows, out, sub, corr, scale, nm, nf, nb, T.dev.tw, st);
             }
+            TC_TRY(lists_match());
             switch (sl.ts) {
                 case 16: TC_TRY((spread_pass<R, 16, true>(cpts, geo, sl, es, nb, grid, st))); break;
                 case 32: TC_TRY((spread_pass<R, 32, true>(cpts, geo, sl, es, nb, grid, st))); break;
@@ -1330,6 +1334,7 @@ static int t1_from_points(const cpx<R> *cpts, const PolarDev &geo, const SpreadL
             return t1_fast_fft(grid, rows, out, sub, corr, scale, nm, nf, nb, T.dev.tw, st);
         }
     }
+    TC_TRY(lists_match());
     switch (sl.ts) {
         case 16: TC_TRY((spread_pass<R, 16>(cpts, geo, sl, es, nb, grid, st))); break;
         case 32: TC_TRY((spread_pass<R, 32>(cpts, geo, sl, es, nb, grid, st))); break;
@@ -1624,7 +1629,8 @@ int psf_fp64(Plan &pl, const std::vector<double> &cs, const std::vector<double> 
 }
 
 // ---------------------------------------------------------------------------
-// spread autotuner.  The type-1 spreading (back-projection, NUFFT gradient)
+// spread autotuner of the tile path (general engine, or kernel widths above
+// 8).  The type-1 spreading (back-projection, NUFFT gradient)
 // splits the fine grid into TS x TS tiles, each accumulated in shared memory
 // by one CTA per sub-problem of at most max_points points.  Small tiles cut
 // the shared-memory footprint and the write-out; large tiles cut the number
