@@ -48,15 +48,21 @@ k_mbir_update(float *__restrict__ X, const float *__restrict__ H, const float *_
                       use_tma ? &tmap : nullptr);
 }
 
-// Planes per CTA of the update: where the tiles alone leave CTA slots idle
-// the volume is split in z, at multiples of the slices summed in FP32 (so the
-// split does not change what is summed).  A run costs its planes, one more
-// for the plane below it and about one of start-up; the split with the
-// smallest (waves of CTAs) x (planes per CTA) is taken.  Update of 24 slices
-// of 300^2 (50 tiles for 296 slots; runs of 8) 0.165 -> 0.084 ms, of 64 x
-// 128^2 0.379 -> 0.066, of 33 x 500^2 0.224 -> 0.177; 16 x 1024^2 and larger
-// volumes keep one run.
-static int update_run(int tiles, int S, int slots) {
+// Planes per CTA of the update: where the tiles alone leave CTA slots idle,
+// in the only wave or in the last one, the volume is split in z, at multiples
+// of the slices summed in FP32 (so the split does not change what is summed).
+// A run costs its planes, one more for the plane below it and about one of
+// start-up; the split with the smallest (waves of CTAs) x (planes per CTA) is
+// taken.  Update, one run -> split, ms: 24 slices of 300^2 (50 tiles for 296
+// slots; runs of 8) 0.165 -> 0.084, 64 x 128^2 0.379 -> 0.066, 64 x 512^2
+// (runs of 32) 0.401 -> 0.274, 256 x 1024^2 (64) 3.81 -> 3.26, 96 x 1400^2
+// (32) 2.54 -> 2.37, 256 x 2908^2 (64) 26.16 -> 25.77.  Of about 60 shapes
+// the split was more than 0.2 % slower than one run at three, where the model
+// expects 2 % or less: 16 x 1200^2 0.349 -> 0.352, 16 x 1206^2 0.398 -> 0.401,
+// 48 x 2112^2 2.604 -> 2.626; the same margin gives 16 x 1120^2 7 % and
+// 96 x 2908^2 0.8 %, and a finer model of the last wave lost at some shapes
+// what it gained at others.
+int update_run(int tiles, int S, int slots) {
     int best = S;
     double cost = (double)ceil_div(tiles, slots) * (S + 1.0);
     for (int zc = ACC_CHUNK; zc < S; zc += ACC_CHUNK) {

@@ -84,4 +84,8 @@ __device__ __forceinline__ int mbir_decide_core(MbirState *s, const double *u, d
     return cond;
 }
 
+// planes per CTA of the single-volume update: `tiles` tiles of S slices for
+// `slots` resident CTAs (tc_mbir.cu)
+int update_run(int tiles, int S, int slots);
+
 }  // namespace tc
