@@ -16,7 +16,8 @@
 // and the loop runs as one CUDA graph (WHILE node) or from the host.  A scan
 // that has finished (or hit its attempt cap) makes its CTAs return at once.
 // The Toeplitz CTAs pick the register FFT of their scan's size at run time
-// (512 threads: 512 / (M / 16) lines per CTA for every size M = 64 .. 4096).
+// (rows and out 512 threads, columns 256: that over M / 16 lines per CTA for
+// every size M = 64 .. 4096).
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -125,21 +126,19 @@ template <class F>
 __device__ __forceinline__ void bcols(const BScan &d, int q, int pg, c32 *sm) {
     constexpr int L = BColShape<F>::L;
     const int l = threadIdx.x / F::T, t = threadIdx.x % F::T;
-    // with more lines per CTA than columns (M = 64) the surplus lines only
-    // take part in the barriers
+    static_assert(F::M % L == 0, "every line of a CTA is a column");
     const int N = d.N, pos = pg * L + l;
-    const bool valid = pos < F::M;
-    c32 *col = d.W + ((size_t)q * F::M + (valid ? pos : 0)) * d.NS;
+    c32 *col = d.W + ((size_t)q * F::M + pos) * d.NS;
     c32 v[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         v[i] = mk<float>(0.f, 0.f);
         if (!F::low_half(i)) continue;
         const int n = F::nidx(t, i);
-        if (valid && n < N) v[i] = col[n];
+        if (n < N) v[i] = col[n];
     }
     F::template forward<true>(v, sm + l * F::LS, t, d.tw);
-    const float4 *ph = reinterpret_cast<const float4 *>(d.phatp + (size_t)(valid ? pos : 0) * F::M + t * 16);
+    const float4 *ph = reinterpret_cast<const float4 *>(d.phatp + (size_t)pos * F::M + t * 16);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float4 p = __ldg(ph + i);
@@ -154,7 +153,7 @@ __device__ __forceinline__ void bcols(const BScan &d, int q, int pg, c32 *sm) {
     for (int i = 0; i < 16; ++i) {
         if (!F::low_half(i)) continue;
         const int n = F::nidx(t, i);
-        if (valid && n < N) col[n] = v[i];
+        if (n < N) col[n] = v[i];
     }
 }
 
@@ -388,7 +387,7 @@ int mbir_batched(const std::vector<BatchScanIn> &in, int num_iters, int use_grap
                 rows.push_back(make_int4(i, q, rb, 0));
                 outs.push_back(make_int4(i, q, rb, 0));
             }
-            for (int pg = 0; pg < ceil_div(b.M, cols_per_cta(b.M)); ++pg) cols.push_back(make_int4(i, q, pg, 0));
+            for (int pg = 0; pg < b.M / cols_per_cta(b.M); ++pg) cols.push_back(make_int4(i, q, pg, 0));
         }
     }
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
