@@ -76,7 +76,8 @@ constexpr int BT_SMEM = BT_SMEM_C * (int)sizeof(c32);
 // loaded, transformed twice and stored with no other work to hide its memory
 // latency but the other CTAs of the SM.  24 scans of 256^2 .. 1024^2, per
 // attempt: one CTA of 512 threads 365 us; two of 256 (128 registers) 284,
-// three (80 registers, some spilled) 273, four 294.
+// three (80 registers, some spilled) 273, four 294; three without a predicate
+// per line, as it is now, 262.
 constexpr int BCT = 256;
 constexpr int BCOLS = 3;
 template <class F>

@@ -9,10 +9,13 @@ namespace tc {
 // One voxel per thread of a 32 x 8 tile.  Evaluating all 26 edges of every
 // voxel, the kernel ran at the SFU's rate (78 operations per voxel: 317 of
 // its 356 us on 32 slices of 768^2); with shared edges and the ring's 11 %
-// more there are 43, and it takes 272 us (16 x 2048^2: 1246 -> 918).  Now the
-// evaluations' latency bounds it (short-scoreboard and fixed-latency stalls,
-// SFU 64 % busy by its count), and warps per SM count: six CTAs of 40 registers 272 us,
-// five 280, seven (32 registers) 293; 32 x 16 tiles at three CTAs 362.
+// more there are 43, and it takes 272 us (16 x 2048^2: 1246 -> 918).  Now issue
+// bounds it (ncu: 76 % of the slots, SFU pipe 71 %, L1 data pipe 50 %; the
+// waits are for a shared-memory or SFU result), and warps per SM count: six
+// CTAs of 40 registers 272 us, five 280, seven (32 registers) 293; 32 x 16
+// tiles at three CTAs 362.  Volumes of a few hundred thousand voxels take as
+// long as before (10 to 20 us, launch and latency); thin ones whose tiles are
+// mostly padding up to 4 us longer (700 x 3 x 5: 10 -> 14 us).
 constexpr int QTY = 8, QCTAS = 6;
 struct QSmem {
     float plane[3][EdgeTile<QTY>::PN];

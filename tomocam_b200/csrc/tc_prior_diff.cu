@@ -103,8 +103,9 @@ __global__ void k_qggmrf_value(const float *__restrict__ x, int S, int R, int C,
 // evaluated once and passed through shared memory (tc_edges.cuh).  Four
 // buffers of x and v planes: a voxel's backward edges read the plane below.
 // 32 slices of 768^2: 764 -> 562 us, with the two dot products 940 -> 618
-// (one partial pair per run of slices instead of one per slice).  71 KB of
-// shared memory hold it at three CTAs per SM, where latency bounds it.
+// (one partial pair per run of slices instead of one per slice).  Issue bounds
+// it (ncu: 78 % of the slots, L1 data pipe 58 %, FMA pipe 43 %, SFU pipe 37 %)
+// at three CTAs per SM, which both 71 KB of shared memory and 80 registers set.
 constexpr int HTY = 8;
 struct HSmem {
     float x[4][EdgeTile<HTY>::PN], v[4][EdgeTile<HTY>::PN];
